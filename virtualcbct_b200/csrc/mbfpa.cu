@@ -1463,8 +1463,9 @@ __device__ __forceinline__ void march_accumulate(const ProjParams& P, const RayP
 }
 
 // The spectral table in shared memory: bins in pairs, so that the sums over
-// bins run two at a time in packed arithmetic (a last odd bin is paired with
-// one of weight 0).
+// bins run two at a time in packed arithmetic.  A last odd bin is paired with
+// itself, half the weight each: whatever its exponential is (0 behind an
+// infinite path integral, infinite before one of -inf), the pair's sum is the bin's.
 template <int M>
 struct SpecPair {
     f32x2 mu[M];
@@ -1482,10 +1483,8 @@ __device__ __forceinline__ void load_spectrum(const SpectrumDev& sp, SpecPair<M>
     float* dst = reinterpret_cast<float*>(s_sp);
     const int n = (sp.NE + 1) / 2 * W;
     for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < n; i += blockDim.x * blockDim.y) {
-        const int e = 2 * (i / W) + (i & 1), k = (i % W) >> 1;
-        float v = 0.0f;
-        if (e < sp.NE) v = k < M ? mu[8 * e + k] : (k == M ? sp.pdf[e] : 0.0f);
-        dst[i] = v;
+        const int e0 = 2 * (i / W), e = min(e0 + (i & 1), sp.NE - 1), k = (i % W) >> 1;
+        dst[i] = k < M ? mu[8 * e + k] : (k == M ? sp.pdf[e] * (e0 + 1 < sp.NE ? 1.0f : 0.5f) : 0.0f);
     }
 }
 
@@ -1511,7 +1510,8 @@ __device__ __forceinline__ f32x2 exp2_2(f32x2 x)
 // sum_E pdf_E exp(-sum_k mu_k(E) L_k).  The exponents are formed for base 2 from
 // path integrals scaled by -log2 e (rounded once per ray and element, as L
 // itself is), so that a bin's exponential is one instruction.  Where a bin falls
-// below 2^-126 the sum is done again with expf, which keeps what it can there.
+// below 2^-126, or the sum is not finite (a path integral that only its scaling
+// takes beyond the largest float), it is done again with expf and L as it is.
 template <int M>
 __device__ __forceinline__ float spectral_sum(const SpecPair<M>* s_sp, int NE, const float* L)
 {
@@ -1532,7 +1532,8 @@ __device__ __forceinline__ float spectral_sum(const SpecPair<M>* s_sp, int NE, c
         acc = ffma2(q.pdf, exp2_2(x), acc);
     }
     float a, b;
-    if (!(lo > -125.0f)) {
+    f2unpack(acc, a, b);
+    if (!(lo > -125.0f && fabsf(a + b) < kInf)) {
         acc = 0ull;
 #pragma unroll
         for (int k = 0; k < M; k++) L2[k] = f2pack(L[k], L[k]);
@@ -1542,8 +1543,8 @@ __device__ __forceinline__ float spectral_sum(const SpecPair<M>* s_sp, int NE, c
             f2unpack(attenuation2<M>(q, L2), a, b);
             acc = ffma2(q.pdf, f2pack(expf(-a), expf(-b)), acc);
         }
+        f2unpack(acc, a, b);
     }
-    f2unpack(acc, a, b);
     return a + b;
 }
 
