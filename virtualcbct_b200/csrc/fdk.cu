@@ -584,7 +584,7 @@ cudaError_t launch_filter_direct(const float* proj, float* out, const float* hT,
     const int widest = (a.groups + a.npass - 1) / a.npass;
     const size_t smem = ((size_t)a.kc * FT_LD + (size_t)2 * FT_K * 32 * widest) * sizeof(float);
     auto k = widest <= 2 ? filter_direct_kernel<2> : filter_direct_kernel<FT_TN>;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<dim3((unsigned)rows, (unsigned)((a.npass + a.per - 1) / a.per)), 256, smem, st>>>(a);
     return cudaGetLastError();

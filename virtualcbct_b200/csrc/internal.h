@@ -20,6 +20,20 @@ int cuda_fail(cudaError_t e, const char* what);
         if (e__ != cudaSuccess) return ::vcbct::cuda_fail(e__, #call); \
     } while (0)
 
+// A launch whose blocks take more than 48 KB of dynamic shared memory needs its
+// kernel's limit raised.  The limit is the kernel's (on a device), shared by
+// every host thread and by launches prepared long before, so it is only ever
+// set to `most`, what the kernel's largest launch takes, never to one call's
+// size: that would lower it under another call's launch.
+constexpr size_t kSmemDefault = 48 * 1024, kSmemMost = 227 * 1024;
+template <class K>
+cudaError_t allow_smem(K kernel, size_t bytes, size_t most = kSmemMost)
+{
+    if (bytes > most) return cudaErrorInvalidValue;
+    if (bytes <= kSmemDefault) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Per-view geometry the projector kernels read (double, from the host
 // tables of prepareTrigonometricTable, misc.cpp:10-37).
 struct ViewGeom {

@@ -2175,10 +2175,8 @@ static cudaError_t launch_fwd_t(const ForwardArgs& a, cudaStream_t st)
     dim3 grid((a.p.W + cpb - 1) / cpb, a.p.V, a.nbands > 0 ? a.nbands : (a.p.H + 31) / 32);
     const size_t shm = block_smem<M>(a.spec.NE, cpb, true, MODE != kWalk);
     auto k = forward_kernel<M, COUNT, MODE, U16>;
-    if (shm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(k, shm);
+    if (e != cudaSuccess) return e;
     k<<<grid, block, shm, st>>>(a);
     return cudaGetLastError();
 }
@@ -2239,9 +2237,8 @@ int batch_blocks_per_sm(const BatchShape& s)
 {
     const BatchKernels k = batch_kernels(s);
     int n = 0;
-    if (k.shm > 48 * 1024 &&
-        (cudaFuncSetAttribute(k.persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.shm) != cudaSuccess ||
-         cudaFuncSetAttribute(k.flat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.shm) != cudaSuccess))
+    // (the persistent kernel holds its tile's number in static shared memory)
+    if (allow_smem(k.persistent, k.shm, kSmemMost - 1024) != cudaSuccess || allow_smem(k.flat, k.shm) != cudaSuccess)
         return 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.persistent, 32 * s.cols_per_block, k.shm);
     return n;
@@ -2315,10 +2312,8 @@ static cudaError_t launch_adj_t(const AdjointArgs& a, cudaStream_t st)
     dim3 grid((a.p.W + cpb - 1) / cpb, a.p.V, (a.p.H + 31) / 32);
     const size_t shm = block_smem<M>(a.spec.NE, cpb, !STATE, COL, STATE ? sizeof(ScatterTab<M>) : sizeof(ColTab<M>));
     auto k = adjoint_kernel<M, STATE, COL>;
-    if (shm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(k, shm);
+    if (e != cudaSuccess) return e;
     k<<<grid, block, shm, st>>>(a);
     return cudaGetLastError();
 }

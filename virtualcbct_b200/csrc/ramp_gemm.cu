@@ -746,7 +746,7 @@ cudaError_t launch_ramp_gemm_bf16x3(const float* proj, float* out, const float* 
     if (W < 16 || W > 4096) return cudaErrorInvalidValue;
     const bool fused = ramp_gemm_fused(proj, out, W);
     const Layout L = layout_for(V, H, W, fused);
-    if (L.smem > 227 * 1024) return cudaErrorInvalidValue;
+    if (L.smem > kSmemMost) return cudaErrorInvalidValue;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     __nv_bfloat16* bp = reinterpret_cast<__nv_bfloat16*>(ws + L.b_off);
     int* err = reinterpret_cast<int*>(ws + L.err_off);
@@ -776,11 +776,11 @@ cudaError_t launch_ramp_gemm_bf16x3(const float* proj, float* out, const float* 
     GemmArgs g{out, views, fused ? wts : nullptr, pitch, sad, L.M, H, W, L.NT, L.Kp, L.Kp / BK, vec, err};
     const dim3 grid((L.M + BM - 1) / BM, L.ntiles);
     if (fused) {
-        e = cudaFuncSetAttribute(ramp_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+        e = allow_smem(ramp_gemm_kernel<true>, L.smem);
         if (e != cudaSuccess) return e;
         ramp_gemm_kernel<true><<<grid, kThreads, L.smem, st>>>(tmA, tmB, tmO, g);
     } else {
-        e = cudaFuncSetAttribute(ramp_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+        e = allow_smem(ramp_gemm_kernel<false>, L.smem);
         if (e != cudaSuccess) return e;
         ramp_gemm_kernel<false><<<grid, kThreads, L.smem, st>>>(tmA, tmB, tmO, g);
     }
