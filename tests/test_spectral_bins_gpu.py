@@ -50,6 +50,22 @@ def test_rays_through_an_infinite_voxel_are_dark_and_scatter_nothing(cuda, bins,
         assert np.linalg.norm(d) <= 1e-5 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("xfactor", [1000.0, 40.0, 15.0])  # all sums above the floor; most; few
+def test_a_heavy_spectrum_keeps_its_weakest_sums(cuda, xfactor):
+    """Which sums are done again follows the spectrum's own weight, here 2^30."""
+    g, tabs, vol, mu, pdf, p = _case(90, 64)
+    p.load_volume_f32(vol)
+    pdf = pdf * np.float32(2.0 ** 30)
+    p.set_spectrum(mu, pdf, xfactor)
+    got = p.forward().cpu().numpy().astype(np.float64) / 2.0 ** 30
+    ref = O.mbfpa_forward(g, tabs, None, mu, pdf, xfactor, volf=vol, exact=True, want=("d",))["d"] / 2.0 ** 30
+    ok = ref > 1e-36
+    # a float exponent T is off by a few of its last places: the path
+    # integrals (1e-7 each), the products and the scaling
+    T = 1.0 - np.log(ref[ok])
+    assert ok.any() and (np.abs(got[ok] - ref[ok]) <= (16 * T + 40) * 2.0 ** -24 * ref[ok]).all()
+
+
 @pytest.mark.parametrize("bins", [89, 90])
 def test_finite_path_integrals_near_the_largest_float(cuda, bins):
     """An element without attenuation whose path integrals are finite, but not

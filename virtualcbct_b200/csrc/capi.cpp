@@ -85,7 +85,7 @@ struct vcbct_projector {
     DevBuf vol;        // packed volume, either form, room for the f32 form (its address never changes)
     DevBuf stage;      // staging for host inputs / outputs
     DevBuf spec_mu;    // float4 [NE][2]
-    DevBuf spec_pdf;   // float [NE]
+    DevBuf spec_pdf;   // float [1 + NE]
     DevBuf grad_pk;    // packed float gradient accumulator
     DevBuf counter;    // unsigned long long, int err flag, [16]: int form of `vol`
     int* form() const { return reinterpret_cast<int*>(counter.as<char>() + 16); }
@@ -222,9 +222,11 @@ extern "C" int vcbct_projector_set_spectrum(vcbct_projector* p, const float* mu,
         for (int k = 0; k < p->g.num_material; k++)
             tab[(size_t)e * 8 + k] = (float)((double)mu[(size_t)k * NE + e] / xfactor);
     VCBCT_CUDA_TRY(p->spec_mu.ensure(tab.size() * sizeof(float)));
-    VCBCT_CUDA_TRY(p->spec_pdf.ensure((size_t)NE * sizeof(float)));
+    std::vector<float> weights(pdf, pdf + NE);
+    weights.insert(weights.begin(), spectral_floor(pdf, NE));
+    VCBCT_CUDA_TRY(p->spec_pdf.ensure(weights.size() * sizeof(float)));
     VCBCT_CUDA_TRY(cudaMemcpy(p->spec_mu.p, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
-    VCBCT_CUDA_TRY(cudaMemcpy(p->spec_pdf.p, pdf, (size_t)NE * sizeof(float), cudaMemcpyHostToDevice));
+    VCBCT_CUDA_TRY(cudaMemcpy(p->spec_pdf.p, weights.data(), weights.size() * sizeof(float), cudaMemcpyHostToDevice));
     p->NE = NE;
     return VCBCT_OK;
 }

@@ -73,12 +73,19 @@ cudaError_t launch_pack_u16(const uint16_t* src, int N, int nz, int zoff, int Z,
 cudaError_t launch_pack_f32(const float* src, int N, int Z, int nmat, float4* dst, int* form, cudaStream_t st);
 cudaError_t launch_unpack_grad(const float* planes, int N, int Z, int nmat, float* dst, cudaStream_t st);
 
-// Spectral table: per bin 8 floats mu_k(E)/xfactor (zero padded) + pdf.
+// Spectral table: per bin 8 floats mu_k(E)/xfactor (zero padded) + pdf, and
+// before the first bin's pdf the spectrum's floor: 2^-100 of its weight.
 struct SpectrumDev {
     const float4* mu8;  // [NE][2] float4
-    const float* pdf;   // [NE]
+    const float* pdf;   // [1 + NE]
     int NE;
 };
+inline float spectral_floor(const float* pdf, int NE)
+{
+    double w = 0.0;
+    for (int e = 0; e < NE; e++) w += pdf[e] < 0.0f ? -(double)pdf[e] : (double)pdf[e];
+    return (float)(w * 7.8886090522101181e-31);
+}
 
 struct ForwardArgs {
     ProjParams p;

@@ -1470,7 +1470,7 @@ template <int M>
 struct SpecPair {
     f32x2 mu[M];
     f32x2 pdf;
-    f32x2 pad;  // to a multiple of 16 bytes (M is even)
+    f32x2 floor;  // the spectrum's (it fills the pair to a multiple of 16 bytes: M is even)
 };
 template <int M>
 __host__ __device__ constexpr size_t spec_bytes(int NE) { return (size_t)((NE + 1) / 2) * sizeof(SpecPair<M>); }
@@ -1484,7 +1484,7 @@ __device__ __forceinline__ void load_spectrum(const SpectrumDev& sp, SpecPair<M>
     const int n = (sp.NE + 1) / 2 * W;
     for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < n; i += blockDim.x * blockDim.y) {
         const int e0 = 2 * (i / W), e = min(e0 + (i & 1), sp.NE - 1), k = (i % W) >> 1;
-        dst[i] = k < M ? mu[8 * e + k] : (k == M ? sp.pdf[e] * (e0 + 1 < sp.NE ? 1.0f : 0.5f) : 0.0f);
+        dst[i] = k < M ? mu[8 * e + k] : (k == M ? sp.pdf[1 + e] * (e0 + 1 < sp.NE ? 1.0f : 0.5f) : sp.pdf[0]);
     }
 }
 
@@ -1509,14 +1509,18 @@ __device__ __forceinline__ f32x2 exp2_2(f32x2 x)
 
 // sum_E pdf_E exp(-sum_k mu_k(E) L_k).  The exponents are formed for base 2 from
 // path integrals scaled by -log2 e (rounded once per ray and element, as L
-// itself is), so that a bin's exponential is one instruction.  Where a bin falls
-// below 2^-126, or the sum is not finite (a path integral that only its scaling
-// takes beyond the largest float), it is done again with expf and L as it is.
+// itself is), so that a bin's exponential is one instruction.  A bin below 2^-126
+// counts as 0, at most 2^-126 of the spectrum's weight in all: from a sum of
+// 2^-100 of it (the floor) on that is below a quarter of its last place.  A sum
+// under the floor, or one that is not finite (a path integral that only its
+// scaling takes beyond the largest float), is done again with expf and L as it is.
+// Asking every bin instead did most sums of a body twice: 10 keV bins behind
+// 20 cm of water are below 2^-126 (48 phantoms of 64x64xZ: 0.321 -> 0.284 ms; 256x256x100, 60 views of
+// 200 x 200: 1.54 -> 1.44).
 template <int M>
 __device__ __forceinline__ float spectral_sum(const SpecPair<M>* s_sp, int NE, const float* L)
 {
     f32x2 L2[M], acc = 0ull;
-    float lo = 0.0f;
 #pragma unroll
     for (int k = 0; k < M; k++) {
         const float l = L[k] * -1.4426950408889634f;
@@ -1525,15 +1529,12 @@ __device__ __forceinline__ float spectral_sum(const SpecPair<M>* s_sp, int NE, c
 #pragma unroll 2
     for (int e = 0; e < (NE + 1) / 2; e++) {
         const SpecPair<M> q = s_sp[e];
-        const f32x2 x = attenuation2<M>(q, L2);
-        float a, b;
-        f2unpack(x, a, b);
-        lo = fminf(lo, fminf(a, b));
-        acc = ffma2(q.pdf, exp2_2(x), acc);
+        acc = ffma2(q.pdf, exp2_2(attenuation2<M>(q, L2)), acc);
     }
-    float a, b;
+    float a, b, floor, unused;
     f2unpack(acc, a, b);
-    if (!(lo > -125.0f && fabsf(a + b) < kInf)) {
+    f2unpack(s_sp->floor, floor, unused);
+    if (!(a + b >= floor && a + b < kInf)) {
         acc = 0ull;
 #pragma unroll
         for (int k = 0; k < M; k++) L2[k] = f2pack(L[k], L[k]);

@@ -27,7 +27,7 @@ constexpr size_t kOffRaw = 0;                 // caller's cos/sin/Xc/Yc: 4 x V d
 constexpr size_t kOffViews = 128 * 1024;      // ViewGeom[V] built from them (<= 32 KiB)
 constexpr size_t kOffMuRaw = 160 * 1024;      // caller's mu [nmat][NE] floats (<= 32 KiB)
 constexpr size_t kOffMu8 = 192 * 1024;        // [NE][8] floats mu / xfactor (<= 32 KiB)
-constexpr size_t kOffPdf = 224 * 1024;        // [NE] floats (<= 4 KiB)
+constexpr size_t kOffPdf = 224 * 1024;        // [1 + NE] floats (<= 4 KiB + 4)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -120,11 +120,13 @@ extern "C" int vcbct_mbfpa_forward_noalloc(const vcbct_proj_geometry* g, const d
         std::memcpy(hraw + 2 * V, xcenter_shift, sizeof(double) * V);
         std::memcpy(hraw + 3 * V, ycenter_shift, sizeof(double) * V);
         std::memcpy(g_host_stage + kOffMuRaw, attenuation, sizeof(float) * nmat * NE);
-        std::memcpy(g_host_stage + kOffPdf, pdf, sizeof(float) * NE);
+        const float floor = spectral_floor(pdf, NE);
+        std::memcpy(g_host_stage + kOffPdf, &floor, sizeof(float));
+        std::memcpy(g_host_stage + kOffPdf + sizeof(float), pdf, sizeof(float) * NE);
         VCBCT_CUDA_TRY(cudaMemcpyAsync(raw, hraw, sizeof(double) * 4 * V, cudaMemcpyHostToDevice, st));
         VCBCT_CUDA_TRY(cudaMemcpyAsync(mu_raw, g_host_stage + kOffMuRaw, sizeof(float) * nmat * NE,
                                        cudaMemcpyHostToDevice, st));
-        VCBCT_CUDA_TRY(cudaMemcpyAsync(dpdf, g_host_stage + kOffPdf, sizeof(float) * NE, cudaMemcpyHostToDevice,
+        VCBCT_CUDA_TRY(cudaMemcpyAsync(dpdf, g_host_stage + kOffPdf, sizeof(float) * (1 + NE), cudaMemcpyHostToDevice,
                                        st));
     }
     build_views_kernel<<<(V + 127) / 128, 128, 0, st>>>(raw, V, views);
