@@ -170,7 +170,9 @@ int vcbct_projector_adjoint_state(vcbct_projector* p, const float* d_L, const fl
  * projects all of them either in one persistent launch that balances the
  * uneven work through a global tile counter, as per-item launches on two
  * branches forked from `stream`, or in one flat launch with a block per tile
- * of every item (the default; vcbct_batch_autotune picks the fastest);
+ * of every item (the default; vcbct_batch_autotune picks the fastest; items
+ * that run different kernels, by their geometry and their volume's type, go in
+ * launches of their own, and those whose rays share columns always flat);
  * with use_graph != 0 the launch sequence
  * is captured into a CUDA graph on the first call and replayed on later calls
  * (the items must not change in between; adding an item rebuilds it). */

@@ -102,3 +102,34 @@ def test_projector_autotune_keeps_results(cuda):
     c = p.autotune()
     assert c in (2, 4, 8)
     assert np.max(np.abs(p.forward().cpu().numpy() - ref) / ref) <= 1e-6
+
+
+@pytest.mark.parametrize("strategy", [Batch.PERSISTENT, Batch.PER_ITEM, Batch.FLAT])
+def test_items_of_every_kind(cuda, strategy):
+    """Walked and by shared columns (H), uint16 and float volumes in turn, 46
+    items (more than a launch holds of one kind); then with every volume's type
+    the other way round, by the launches already prepared."""
+    import torch
+    ps, b = [], Batch()
+    for i in range(46):
+        g, tabs, vol, _ = proj_case("random", seed=200 + i, N=16 + i % 3, Z=4 + i % 5, V=1 + i % 2, W=8 + i % 4,
+                                    H=96 if i % 23 == 1 else 6)
+        mu, pdf = spectrum()
+        p = Projector(g, *tabs)
+        p.set_spectrum(mu, pdf, 1000.0)
+        ps.append((p, vol))
+    for turn in (0, 1):
+        plain = []
+        for i, (p, vol) in enumerate(ps):
+            (p.load_volume if (i % 7 != 0) != bool(turn) else lambda v: p.load_volume_f32(v.astype(np.float32)))(vol)
+            plain.append(p.forward().cpu().numpy())
+        if turn == 0:
+            outs = [b.add(p) for p, _ in ps]
+            b.configure(strategy, 2)
+        for use_graph in (True, False):
+            for o in outs:
+                o.fill_(float("nan"))
+            b.forward(use_graph=use_graph)
+            torch.cuda.synchronize()
+            for o, ref in zip(outs, plain):
+                assert np.array_equal(o.cpu().numpy(), ref), (turn, use_graph)

@@ -881,15 +881,17 @@ extern "C" void vcbct_IR_ImageCBCT(const int ite, int reconSize, int reconSlices
 // vcbct_batch_autotune picks another (48 phantoms of 64x64xZ, 8-24 views of
 // 32x32: flat 0.31 ms, persistent 0.38, whose loop keeps state across the
 // march that costs it registers):
-//  - persistent: one launch of persistent_batch_kernel per kFlatItems items,
-//    a GPU-filling grid whose blocks take every item's tiles from a counter
-//    (counter reset + kernel);
+//  - persistent: one launch of persistent_batch_kernel per kFlatItems walked
+//    items, a GPU-filling grid whose blocks take every item's tiles from a
+//    counter (counter reset + kernel); items summed by shared columns go as in
+//    the flat strategy (a loop around that march spills: 40 items of 128x128xZ
+//    with 64x96 detectors 5.22 ms persistent, 3.42 flat);
 //  - per-item: each item's own forward_kernel launch, spread over two
 //    branches that fork from and join to the caller's stream, so one item's
 //    tail overlaps the next item's start;
 //  - flat: one launch of flat_batch_kernel with a block per tile of every
-//    item (up to kFlatItems items per launch, their arguments in the
-//    launch's parameter block).
+//    item of a kind (up to kFlatItems items per launch, their arguments in
+//    the launch's parameter block).
 // Either launch sequence is captured once into a CUDA graph and replayed.
 
 constexpr int kBatchBranches = 2;
@@ -899,11 +901,14 @@ struct vcbct_batch {
     std::vector<vcbct_projector*> proj;
     std::vector<float*> outs;
     DevBuf counter;
-    long long total = 0;
-    BatchShape shape{};
-    int cols_per_block = 4, blocks = 0;
+    int cols_per_block = 4;
     int strategy = 2;   // 0: persistent launch, 1: per-item launches, 2: single flat launch
-    std::vector<FlatBatch> flat;  // strategies 0 and 2: the launches' parameter blocks
+    struct Launch {     // strategies 0 and 2: up to kFlatItems items of one kind
+        FlatBatch b;
+        BatchShape shape;
+        int blocks;     // of the persistent launch
+    };
+    std::vector<Launch> flat;
     bool dirty = true;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -967,47 +972,50 @@ extern "C" int vcbct_batch_configure(vcbct_batch* b, int strategy, int cols_per_
 static int batch_build(vcbct_batch* b)
 {
     if (b->proj.empty()) return fail(VCBCT_ERR_STATE, "empty batch");
-    b->shape = BatchShape{};
-    b->shape.cols_per_block = b->cols_per_block;
-    size_t n_u16 = 0, n_col = 0;
-    b->total = 0;
     const int cpb = b->cols_per_block;
-    // parameter blocks of the single-launch strategies, kFlatItems items each
-    b->flat.clear();
-    for (size_t i0 = 0; i0 < b->proj.size(); i0 += kFlatItems) {
-        FlatBatch fb{};
-        const size_t n = std::min<size_t>(kFlatItems, b->proj.size() - i0);
-        fb.nitems = (int)n;
-        long long t = 0;
-        for (size_t i = 0; i < n; i++) {
-            vcbct_projector* p = b->proj[i0 + i];
-            ForwardArgs a;
-            int rc = make_fwd_args(p, a);
-            if (rc) return rc;
-            a.out = b->outs[i0 + i];
-            a.cols_per_block = cpb;
-            fb.fa[i] = a;
-            fb.ncolb[i] = (p->g.proj_width + cpb - 1) / cpb;
-            fb.begin[i] = t;
-            t += (long long)fb.ncolb[i] * p->g.n_views * ((p->g.proj_height + 31) / 32);
-            b->shape.columns |= a.columns != 0;
-            n_col += a.columns != 0;
-            n_u16 += a.vol.expect == kFormU16;
-            b->shape.NEmax = std::max(b->shape.NEmax, p->NE);
-            b->shape.nmat_max = std::max(b->shape.nmat_max, p->g.num_material);
-        }
-        fb.begin[n] = t;
-        b->total += t;
-        b->flat.push_back(fb);
-    }
-    VCBCT_CUDA_TRY(b->counter.ensure(64));
     int dev = 0, sms = 0;
     VCBCT_CUDA_TRY(cudaGetDevice(&dev));
     VCBCT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    b->shape.u16 = 2 * n_u16 >= b->proj.size();
-    b->shape.all_columns = n_col == b->proj.size();
-    const int per_sm = batch_blocks_per_sm(b->shape);
-    b->blocks = std::max(1, per_sm) * sms;
+    // The launches of the single-launch strategies: items of a kind (walked or
+    // summed by shared columns, uint16 or float records) go together, so that
+    // each runs the kernel made for it.  One kernel for both kinds reserves the
+    // columns' registers and tables for the walk too: 48 items, half of them
+    // walked (128x128xZ) and half by columns (96x96xZ), flat 2.60 -> 2.10 ms.
+    b->flat.clear();
+    for (const int kind : {0, 1, 2, 3}) {
+        const bool columns = kind & 2, u16 = kind & 1;
+        std::vector<size_t> items;
+        for (size_t i = 0; i < b->proj.size(); i++)
+            if (march_shares_columns(b->proj[i]->pp) == columns && (b->proj[i]->have_u16 != 0) == u16) items.push_back(i);
+        for (size_t i0 = 0; i0 < items.size(); i0 += kFlatItems) {
+            b->flat.emplace_back();
+            auto& [fb, shape, blocks] = b->flat.back();
+            fb = FlatBatch{};
+            shape = BatchShape{};
+            shape.columns = columns;
+            shape.u16 = u16;
+            shape.cols_per_block = cpb;
+            const int n = (int)std::min<size_t>(kFlatItems, items.size() - i0);
+            fb.nitems = n;
+            long long t = 0;
+            for (int i = 0; i < n; i++) {
+                vcbct_projector* p = b->proj[items[i0 + i]];
+                ForwardArgs& a = fb.fa[i];
+                const int rc = make_fwd_args(p, a);
+                if (rc) return rc;
+                a.out = b->outs[items[i0 + i]];
+                a.cols_per_block = cpb;
+                fb.ncolb[i] = (p->g.proj_width + cpb - 1) / cpb;
+                fb.begin[i] = t;
+                t += (long long)fb.ncolb[i] * p->g.n_views * ((p->g.proj_height + 31) / 32);
+                shape.NEmax = std::max(shape.NEmax, p->NE);
+                shape.nmat_max = std::max(shape.nmat_max, p->g.num_material);
+            }
+            fb.begin[n] = t;
+            blocks = std::max(1, batch_blocks_per_sm(shape)) * sms;
+        }
+    }
+    VCBCT_CUDA_TRY(b->counter.ensure(64));
     batch_drop_graph(b);
     b->dirty = false;
     return VCBCT_OK;
@@ -1016,13 +1024,16 @@ static int batch_build(vcbct_batch* b)
 static int batch_launch(vcbct_batch* b, cudaStream_t st)
 {
     if (b->strategy == 2) {
-        for (const FlatBatch& fb : b->flat)
-            VCBCT_CUDA_TRY(launch_flat_batch(fb, b->shape, st));
+        for (const auto& l : b->flat) VCBCT_CUDA_TRY(launch_flat_batch(l.b, l.shape, st));
         return VCBCT_OK;
     }
     if (b->strategy == 0) {
-        for (const FlatBatch& fb : b->flat)
-            VCBCT_CUDA_TRY(launch_persistent_batch(fb, b->shape, b->blocks, b->counter.as<unsigned long long>(), st));
+        for (const auto& l : b->flat) {
+            if (l.shape.columns)
+                VCBCT_CUDA_TRY(launch_flat_batch(l.b, l.shape, st));
+            else
+                VCBCT_CUDA_TRY(launch_persistent_batch(l.b, l.shape, l.blocks, b->counter.as<unsigned long long>(), st));
+        }
         return VCBCT_OK;
     }
     if (!b->fork) {

@@ -125,16 +125,16 @@ struct FlatBatch {
     long long begin[kFlatItems + 1];  // first tile of each item; begin[nitems] = total
     ForwardArgs fa[kFlatItems];
 };
+// Of the items of one launch, which are of one kind.
 struct BatchShape {
     int NEmax, nmat_max;
-    bool columns, u16;   // an item is summed by shared columns; most items hold uint16 values
-    bool all_columns;    // every item is
+    bool columns, u16;   // summed by shared columns; uint16 records
     int cols_per_block;
 };
 cudaError_t launch_flat_batch(const FlatBatch& b, const BatchShape& s, cudaStream_t st);
 
-// The same items in one persistent launch of `blocks` blocks that take work
-// tiles from `counter` (zeroed by the launch).
+// The same items, which are walked, in one persistent launch of `blocks` blocks
+// that take work tiles from `counter` (zeroed by the launch).
 cudaError_t launch_persistent_batch(const FlatBatch& b, const BatchShape& s, int blocks, unsigned long long* counter,
                                     cudaStream_t st);
 int batch_blocks_per_sm(const BatchShape& s);

@@ -1441,9 +1441,8 @@ __device__ __forceinline__ void scatter_columns(const ProjParams& P, const RayPl
     }
 }
 
-// How a kernel sums along its rays: each ray on its own, by shared columns,
-// or as the item says (batches).
-enum { kWalk = 0, kColumns = 1, kEither = 2 };
+// How a kernel sums along its rays: each ray on its own, or by shared columns.
+enum { kWalk = 0, kColumns = 1 };
 
 // Two-level summation: the visitor accumulates into its pair sums; every 32 iterations
 // the partials are folded into L (bounds the FP32 error growth).
@@ -1603,7 +1602,7 @@ __device__ __forceinline__ void warp_range_k(int klo, int khi, bool use, int& Kl
 // [Klo, Khi]).  The interval march is used unless a lane of the warp has
 // |Z1| >= 1 (more than one z plane per step), where the per-step march keeps
 // the reference's last-plane-only split.  R.active is warp-uniform.
-// tab: the warp's column table, nullptr: walk every ray on its own.
+// tab: the warp's column table (kColumns).
 template <class Acc, int M, int MODE>
 __device__ __forceinline__ void ray_integrals(const ProjParams& P, const RayPlan& R, bool act, int Klo, int Khi,
                                               IvRec* wbuf, Acc& acc, ColTab<M>* tab)
@@ -1624,7 +1623,7 @@ __device__ __forceinline__ void ray_integrals(const ProjParams& P, const RayPlan
     };
     const XyPlan& xp = publish_plan<MODE != kWalk>(R, wbuf);
     if (Klo <= Khi) {
-        if (MODE == kColumns || (MODE == kEither && tab))
+        if constexpr (MODE == kColumns)
             march_columns<Acc, M>(P, R, xp, act, Klo, Khi, wbuf, tab, acc, fold);
         else
             march_intervals(P, R, xp, act, Klo, Khi, wbuf, acc, fold);
@@ -1675,7 +1674,7 @@ __device__ __forceinline__ void forward_tile_of(const ForwardArgs& a, const Spec
     unsigned nseg = 0;
     float* s_L = reinterpret_cast<float*>(s_iv + blockDim.y * kSlots) + threadIdx.y * 32 + lane;
     ColTab<M>* tab = nullptr;
-    if (MODE == kColumns || (MODE == kEither && a.columns))
+    if (MODE == kColumns)
         tab = reinterpret_cast<ColTab<M>*>(reinterpret_cast<float*>(s_iv + blockDim.y * kSlots) +
                                            M * 32 * blockDim.y) + threadIdx.y;
     nseg = ray_path<M, MODE, U16>(a.vol, P, R, valid, Klo, Khi, wbuf, s_L, tab, L);
@@ -1824,7 +1823,7 @@ __global__ void __launch_bounds__(256, fwd_min_blocks(MODE)) flat_batch_kernel(c
     forward_tile<M, false, MODE, U16>(fa, s_sp, iv_buffer<M>(smem, fa.spec.NE), v, rowt, colb);
 }
 
-// Persistent batched forward projection: a grid of as many blocks as fit on
+// Persistent batched forward projection of walked items: a grid of as many blocks as fit on
 // the GPU at once, every block repeatedly taking the next work tile from a
 // global counter.  Tiles are numbered item by item, and within an item by
 // row band, then view, then column block (the order of forward_kernel's
@@ -1835,9 +1834,9 @@ __global__ void __launch_bounds__(256, fwd_min_blocks(MODE)) flat_batch_kernel(c
 // hold no registers; the walk takes 5 blocks per SM here (64 phantoms of
 // 128x128xZ 7.77 ms, 4 blocks 8.13, 6 8.10); a block reloads the spectrum table only when its next
 // tile belongs to another item.
-template <int M, int MODE, bool U16>
-__global__ void __launch_bounds__(256, MODE == kWalk ? 5 : 3) persistent_batch_kernel(const __grid_constant__ FlatBatch b,
-                                                         unsigned long long* counter, int NEmax)
+template <int M, bool U16>
+__global__ void __launch_bounds__(256, 5) persistent_batch_kernel(const __grid_constant__ FlatBatch b,
+                                                                  unsigned long long* counter, int NEmax)
 {
     extern __shared__ float4 smem[];
     __shared__ long long s_unit;
@@ -1866,7 +1865,7 @@ __global__ void __launch_bounds__(256, MODE == kWalk ? 5 : 3) persistent_batch_k
         const long long rest = w / b.ncolb[lo];
         const int v = (int)(rest % b.fa[lo].p.V);
         const int rowt = (int)(rest / b.fa[lo].p.V);
-        forward_tile<M, false, MODE, U16>(b.fa[lo], s_sp, s_iv, v, rowt, colb);
+        forward_tile<M, false, kWalk, U16>(b.fa[lo], s_sp, s_iv, v, rowt, colb);
         __syncthreads();
     }
 }
@@ -2182,29 +2181,28 @@ static cudaError_t launch_fwd_t(const ForwardArgs& a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// The kernels and the shared memory of a batch: columns alone if every item
-// asks for them, either kind by item if only some do.
+// The kernels and the shared memory of a launch of batch items of one kind.
 struct BatchKernels {
-    void (*persistent)(FlatBatch, unsigned long long*, int);
+    void (*persistent)(FlatBatch, unsigned long long*, int);  // walked items only
     void (*flat)(FlatBatch);
     size_t shm;
 };
-template <int M, int MODE>
-static BatchKernels batch_kernels_of(bool u16, int NEmax, int cpb)
+template <int M, int MODE, bool U16>
+static BatchKernels batch_kernels_of(const BatchShape& s)
 {
-    const size_t shm = block_smem<M>(NEmax, cpb, true, MODE != kWalk);
-    if (u16) return {persistent_batch_kernel<M, MODE, true>, flat_batch_kernel<M, MODE, true>, shm};
-    return {persistent_batch_kernel<M, MODE, false>, flat_batch_kernel<M, MODE, false>, shm};
+    BatchKernels k{nullptr, flat_batch_kernel<M, MODE, U16>, block_smem<M>(s.NEmax, s.cols_per_block, true, MODE != kWalk)};
+    if constexpr (MODE == kWalk) k.persistent = persistent_batch_kernel<M, U16>;
+    return k;
+}
+template <int M>
+static BatchKernels batch_kernels_of(const BatchShape& s)
+{
+    if (s.columns) return s.u16 ? batch_kernels_of<M, kColumns, true>(s) : batch_kernels_of<M, kColumns, false>(s);
+    return s.u16 ? batch_kernels_of<M, kWalk, true>(s) : batch_kernels_of<M, kWalk, false>(s);
 }
 static BatchKernels batch_kernels(const BatchShape& s)
 {
-    if (s.nmat_max <= 6)
-        return s.all_columns ? batch_kernels_of<6, kColumns>(s.u16, s.NEmax, s.cols_per_block)
-               : s.columns   ? batch_kernels_of<6, kEither>(s.u16, s.NEmax, s.cols_per_block)
-                             : batch_kernels_of<6, kWalk>(s.u16, s.NEmax, s.cols_per_block);
-    return s.all_columns ? batch_kernels_of<8, kColumns>(s.u16, s.NEmax, s.cols_per_block)
-           : s.columns   ? batch_kernels_of<8, kEither>(s.u16, s.NEmax, s.cols_per_block)
-                         : batch_kernels_of<8, kWalk>(s.u16, s.NEmax, s.cols_per_block);
+    return s.nmat_max <= 6 ? batch_kernels_of<6>(s) : batch_kernels_of<8>(s);
 }
 
 cudaError_t launch_persistent_batch(const FlatBatch& b, const BatchShape& s, int blocks, unsigned long long* counter,
@@ -2239,7 +2237,8 @@ int batch_blocks_per_sm(const BatchShape& s)
     const BatchKernels k = batch_kernels(s);
     int n = 0;
     // (the persistent kernel holds its tile's number in static shared memory)
-    if (allow_smem(k.persistent, k.shm, kSmemMost - 1024) != cudaSuccess || allow_smem(k.flat, k.shm) != cudaSuccess)
+    if (allow_smem(k.flat, k.shm) != cudaSuccess || !k.persistent ||
+        allow_smem(k.persistent, k.shm, kSmemMost - 1024) != cudaSuccess)
         return 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.persistent, 32 * s.cols_per_block, k.shm);
     return n;
