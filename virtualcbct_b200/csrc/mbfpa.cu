@@ -1823,31 +1823,17 @@ __global__ void __launch_bounds__(256, fwd_min_blocks(MODE)) flat_batch_kernel(c
     forward_tile<M, false, MODE, U16>(fa, s_sp, iv_buffer<M>(smem, fa.spec.NE), v, rowt, colb);
 }
 
-// Persistent batched forward projection of walked items: a grid of as many blocks as fit on
-// the GPU at once, every block repeatedly taking the next work tile from a
-// global counter.  Tiles are numbered item by item, and within an item by
-// row band, then view, then column block (the order of forward_kernel's
-// grid), so the items' uneven view and slice counts load-balance across the
-// whole GPU in one launch.  The items' arguments sit in the launch's
-// parameter block as for flat_batch_kernel: the march reads them from the
-// parameter bank (a block-uniform index found by a binary search), so they
-// hold no registers; the walk takes 5 blocks per SM here (64 phantoms of
-// 128x128xZ 7.77 ms, 4 blocks 8.13, 6 8.10); a block reloads the spectrum table only when its next
-// tile belongs to another item.
-template <int M, bool U16>
-__global__ void __launch_bounds__(256, 5) persistent_batch_kernel(const __grid_constant__ FlatBatch b,
-                                                                  unsigned long long* counter, int NEmax)
+// Tiles of a batch, taken one after another from a counter.
+template <int M, class Tile>
+__device__ __forceinline__ void persistent_tiles(const FlatBatch& b, unsigned long long* counter, SpecPair<M>* s_sp,
+                                                 long long* s_unit, Tile tile)
 {
-    extern __shared__ float4 smem[];
-    __shared__ long long s_unit;
-    SpecPair<M>* s_sp = reinterpret_cast<SpecPair<M>*>(smem);
-    IvRec* s_iv = iv_buffer<M>(smem, NEmax);
     const long long total = b.begin[b.nitems];
     int cur = -1;
     for (;;) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) s_unit = (long long)atomicAdd(counter, 1ull);
+        if (threadIdx.x == 0 && threadIdx.y == 0) *s_unit = (long long)atomicAdd(counter, 1ull);
         __syncthreads();
-        const long long u = s_unit;
+        const long long u = *s_unit;
         if (u >= total) break;  // block-uniform
         int lo = 0, hi = b.nitems - 1;  // last item with begin <= u
         while (lo < hi) {
@@ -1865,9 +1851,51 @@ __global__ void __launch_bounds__(256, 5) persistent_batch_kernel(const __grid_c
         const long long rest = w / b.ncolb[lo];
         const int v = (int)(rest % b.fa[lo].p.V);
         const int rowt = (int)(rest / b.fa[lo].p.V);
-        forward_tile<M, false, kWalk, U16>(b.fa[lo], s_sp, s_iv, v, rowt, colb);
+        tile(b.fa[lo], v, rowt, colb);
         __syncthreads();
     }
+}
+template <int M>
+__device__ __noinline__ void persistent_tiles_any(const FlatBatch& b, unsigned long long* counter, SpecPair<M>* s_sp,
+                                                  IvRec* s_iv, long long* s_unit)
+{
+    persistent_tiles<M>(b, counter, s_sp, s_unit, [&](const ForwardArgs& fa, int v, int rowt, int colb) {
+        if (is_u16(fa.vol)) forward_tile_other<M, false, kWalk, true>(fa, s_sp, s_iv, v, rowt, colb);
+        else forward_tile_other<M, false, kWalk, false>(fa, s_sp, s_iv, v, rowt, colb);
+    });
+}
+
+// Persistent batched forward projection of walked items: a grid of as many
+// blocks as fit on the GPU at once, every block repeatedly taking the next work
+// tile from a global counter.  Tiles are numbered item by item, and within an
+// item by row band, then view, then column block (the order of
+// forward_kernel's grid), so the items' uneven view and slice counts
+// load-balance across the whole GPU in one launch.  The items' arguments sit
+// in the launch's parameter block as for flat_batch_kernel: the march reads them
+// from the parameter bank (a block-uniform index found by a binary search), so
+// they hold no registers; a block reloads the spectrum table only when its next
+// tile belongs to another item.  The loop's state lives across the march: 5
+// blocks per SM (64 phantoms of 128x128xZ 6.99 ms, 4 blocks 7.17, 6 7.54), and a
+// volume of the other form (loaded since the launch was prepared) sends the
+// whole loop to a function of its own, since a call within it would cost every
+// tile the registers it keeps for the caller (7.32 ms).
+template <int M, bool U16>
+__global__ void __launch_bounds__(256, 5) persistent_batch_kernel(const __grid_constant__ FlatBatch b,
+                                                                  unsigned long long* counter, int NEmax)
+{
+    extern __shared__ float4 smem[];
+    __shared__ long long s_unit;
+    SpecPair<M>* s_sp = reinterpret_cast<SpecPair<M>*>(smem);
+    IvRec* s_iv = iv_buffer<M>(smem, NEmax);
+    bool expected = true;
+    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < b.nitems; i += blockDim.x * blockDim.y)
+        expected &= is_u16(b.fa[i].vol) == U16;
+    if (__syncthreads_and(expected))
+        persistent_tiles<M>(b, counter, s_sp, &s_unit, [&](const ForwardArgs& fa, int v, int rowt, int colb) {
+            forward_tile_of<M, false, kWalk, U16>(fa, s_sp, s_iv, v, rowt, colb);
+        });
+    else
+        persistent_tiles_any<M>(b, counter, s_sp, s_iv, &s_unit);
 }
 
 // Register cap of the adjoint (minimum resident 256-thread blocks per SM):
