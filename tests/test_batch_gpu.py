@@ -133,3 +133,24 @@ def test_items_of_every_kind(cuda, strategy):
             torch.cuda.synchronize()
             for o, ref in zip(outs, plain):
                 assert np.array_equal(o.cpu().numpy(), ref), (turn, use_graph)
+
+
+def test_more_tiles_than_a_grid_holds(cuda):
+    """Two items of 1.09e9 one-row tiles: 2.2e9 blocks are more than one launch
+    takes (2^31 - 1)."""
+    import torch
+    ps = []
+    for i in range(2):
+        g, tabs, vol, _ = proj_case("random", seed=i, N=8, Z=2, V=33000, W=33000, H=1,
+                                    angles=np.arange(33000) * (360.0 / 33000))
+        mu, pdf = spectrum()
+        p = Projector(g, *tabs)
+        p.set_spectrum(mu[:, 40:41], pdf[40:41], 1000.0)
+        p.load_volume(vol)
+        ps.append(p)
+    b = Batch()
+    outs = [b.add(p) for p in ps]
+    b.configure(Batch.FLAT, 1)
+    b.forward(use_graph=False)
+    for p, o in zip(ps, outs):
+        assert torch.equal(o, p.forward())

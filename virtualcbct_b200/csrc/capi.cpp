@@ -987,7 +987,7 @@ static int batch_build(vcbct_batch* b)
         std::vector<size_t> items;
         for (size_t i = 0; i < b->proj.size(); i++)
             if (march_shares_columns(b->proj[i]->pp) == columns && (b->proj[i]->have_u16 != 0) == u16) items.push_back(i);
-        for (size_t i0 = 0; i0 < items.size(); i0 += kFlatItems) {
+        for (size_t i0 = 0; i0 < items.size(); i0 += b->flat.back().b.nitems) {
             b->flat.emplace_back();
             auto& [fb, shape, blocks] = b->flat.back();
             fb = FlatBatch{};
@@ -995,22 +995,25 @@ static int batch_build(vcbct_batch* b)
             shape.columns = columns;
             shape.u16 = u16;
             shape.cols_per_block = cpb;
-            const int n = (int)std::min<size_t>(kFlatItems, items.size() - i0);
-            fb.nitems = n;
             long long t = 0;
-            for (int i = 0; i < n; i++) {
-                vcbct_projector* p = b->proj[items[i0 + i]];
-                ForwardArgs& a = fb.fa[i];
+            int n = 0;
+            for (; n < kFlatItems && i0 + n < items.size(); n++) {
+                vcbct_projector* p = b->proj[items[i0 + n]];
+                const int ncolb = (p->g.proj_width + cpb - 1) / cpb;
+                const long long tiles = (long long)ncolb * p->g.n_views * ((p->g.proj_height + 31) / 32);
+                if (n > 0 && t + tiles > INT_MAX) break;  // a grid's limit (one item has at most 2e9)
+                ForwardArgs& a = fb.fa[n];
                 const int rc = make_fwd_args(p, a);
                 if (rc) return rc;
-                a.out = b->outs[items[i0 + i]];
+                a.out = b->outs[items[i0 + n]];
                 a.cols_per_block = cpb;
-                fb.ncolb[i] = (p->g.proj_width + cpb - 1) / cpb;
-                fb.begin[i] = t;
-                t += (long long)fb.ncolb[i] * p->g.n_views * ((p->g.proj_height + 31) / 32);
+                fb.ncolb[n] = ncolb;
+                fb.begin[n] = t;
+                t += tiles;
                 shape.NEmax = std::max(shape.NEmax, p->NE);
                 shape.nmat_max = std::max(shape.nmat_max, p->g.num_material);
             }
+            fb.nitems = n;
             fb.begin[n] = t;
             blocks = std::max(1, batch_blocks_per_sm(shape)) * sms;
         }
