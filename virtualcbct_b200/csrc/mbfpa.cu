@@ -2279,26 +2279,70 @@ cudaError_t launch_band_footprint(const ProjParams& P, const ViewGeom* d_views, 
     return cudaGetLastError();
 }
 
+// What the rules for shared columns look at.
+struct ColumnShape {
+    double rays;    // of a detector column per slice at the isocentre
+    double planes;  // z planes that the detector's steepest ray meets in a batch of steps
+    double inside;  // the same of the steepest ray that stays in the slab, a little less where many rays leave it
+    double slices;  // that a warp's rays meet at the far end of the cylinder
+    bool whole;     // 1 / s is an integer: no dominant-axis plane lies inside a step
+    bool small;     // below 2e6 voxels: gathers hit L1 and L2
+};
+static ColumnShape column_shape(const ProjParams& p)
+{
+    ColumnShape c;
+    const double pitch = p.piso * p.dpn / p.H, half = p.piso * p.dpn / 2.0;
+    const double per_batch = 32.0 * p.s / p.sad / p.step;
+    c.rays = p.step / pitch;
+    c.planes = per_batch * half;
+    const double in_slab = fmin(1.0, p.Z * p.step / 2.0 / half);
+    c.inside = c.planes * in_slab * sqrt(sqrt(in_slab));
+    c.slices = 32.0 * pitch * (1.0 + p.N * p.s / 2.0 / p.sad) / p.step + c.planes + 1.0;
+    c.whole = fabs(1.0 / p.s - rint(1.0 / p.s)) < 1e-6;
+    c.small = (double)p.N * p.N * p.Z < 2e6;
+    return c;
+}
+
+// Enough rays to a slice.  Columns against the walk on B200, times uint16 /
+// float: at 1.15 rays 1.6 / 1.2 (448x448x120) and 1.15-1.2 / 0.94-0.99
+// (256x256x64), at 0.95 0.9-1.15 / 0.8-0.98 everywhere, at 3.1 2.2 / 1.8.  Small
+// volumes also ask that a warp's rays meet no more than 32 slices (batches of steps
+// beyond that fall back to a walk, which small volumes do not repay) unless
+// those inside the slab meet few planes.  Columns / walk, uint16 (float), at 1.15
+// rays and 34-37 slices: 1.31 (1.16) at 0.45 planes (128x128x14), 1.15 (1.03) at
+// 0.83 (128x128x26), 0.87 (0.79) at 1.66 (128x128x52); where 1 / s is not an
+// integer 1.39 (1.30) at 0.6 (96x96x14), 1.16 (1.06) at 1.54 (96x96x36), 0.89 (0.81)
+// at 2.05 (96x96x48).
+static bool rays_share_slices(const ColumnShape& c)
+{
+    return c.rays >= 1.15 && (!c.small || c.slices <= 32.8 || c.inside <= (c.whole ? 0.9 : 1.6));
+}
+
 bool march_shares_columns(const ProjParams& p)
 {
-    // Rays of a detector column per slice at the isocentre (the same line for
-    // both volume forms, whose projections agree bit for bit).  Columns against
-    // the walk on B200, times uint16 / float: at 1.15 rays per slice 1.6 / 1.2
-    // (448x448x120), 1.15-1.2 / 0.94-0.99 (256x256x64), but 1.0 / 0.85
-    // (128x128x48) and 1.1 / 1.0 (64x64x16); at 1.4 1.8 / 1.3, 1.15-1.25 / 1.0,
-    // 1.07 / 0.92 and 1.07 / 1.0; at 0.95 0.9-1.15 / 0.8-0.98 everywhere; at 3.1
-    // 2.2 / 1.8 (448x448x120).
-    // Small volumes (their gathers hit L1 and L2) also ask that a warp's rays
-    // meet no more than 32 slices at the far end of the cylinder: batches beyond
-    // that fall back to the walk and what the columns cost there is not repaid.
-    // Slices met, columns / walk, uint16: 32.1 1.33 (96x96x32), 32.8 1.0
-    // (160x160x90), 33.2 0.75-0.9 (128x128xZ), 35.7 0.83 (100x100x62).
-    const double pitch = p.piso * p.dpn / p.H;
-    if (p.step < 1.15 * pitch) return false;
-    if ((double)p.N * p.N * p.Z >= 2e6) return true;
-    const double planes = 32.0 * p.piso * p.dpn / 2.0 / p.sad * p.s / p.step;
-    const double slices = 32.0 * pitch * (1.0 + p.N * p.s / 2.0 / p.sad) / p.step + planes + 1.0;
-    return slices <= 32.8;
+    // One line for both forms, whose projections agree bit for bit.  A ray's
+    // chunk with a z plane in it costs more here than in the walk, so the more
+    // planes the rays inside the slab meet, the more of them have to share a slice;
+    // the walk pays more for a plane itself where its intervals hold
+    // dominant-axis planes too (1 / s not an integer) or its gathers miss the
+    // caches.  B200, float columns, float walk (uint16 columns, uint16 walk), each
+    // against the walk as it was before there were columns, 60 views of 64 columns:
+    //   whole, 1.15 planes: 0.95, 0.94 (0.85, 1.00) at 1.5 rays (128x128x36)
+    //   whole, 1.54: 1.07, 0.96 (0.97, 1.01) at 1.3, 0.97, 0.92 (0.85, 0.98) at 1.8 (128x128x48)
+    //   whole, 1.54: 0.98, 0.93 (0.81, 0.93) at 1.3 (256x256x96)
+    //   whole, 1.92: 1.15, 0.93 (1.02, 0.95) at 1.3, 1.00, 0.96 (0.87, 1.02) at 1.8 (256x256x120)
+    //   whole, 2.30: 1.10, 0.92 (1.00, 1.00) at 1.8, 0.94, 0.90 (0.85, 0.99) at 2.8 (128x128x72)
+    //   whole, 2.56: 1.14, 0.96 (1.01, 1.02) at 1.8, 1.04, 0.98 (0.92, 1.09) at 2.8 (256x256x160)
+    //   whole, 3.07: 1.12, 0.92 (1.03, 1.03) at 2.2, 1.00, 0.91 (0.90, 1.04) at 3.6 (128x128x96)
+    //   not, 1.84: 0.95, 0.91 (0.87, 0.99) at 1.3 (160x160x72)
+    //   not, 1.94: 0.72, 0.92 (0.68, 1.01) at 1.3 (203x203x96)
+    //   not, 2.46: 1.07, 0.94 (0.96, 1.05) at 1.8, 0.98, 0.93 (0.89, 1.05) at 2.2 (160x160x96)
+    //   not, 3.07: 1.08, 0.92 (1.00, 0.96) at 1.8, 0.96, 0.88 (0.89, 0.97) at 2.2 (64x64x48)
+    const ColumnShape c = column_shape(p);
+    const double least = !c.whole  ? fmin(2.2, 1.15 + 1.5 * (c.inside - 2.0))
+                         : c.small ? 1.15 + 1.35 * (c.inside - 1.3)
+                                   : fmin(2.6, 1.15 + 2.5 * (c.inside - 1.5));
+    return rays_share_slices(c) && c.rays >= least;
 }
 
 bool scatter_shares_columns(const ProjParams& p)
@@ -2309,9 +2353,8 @@ bool scatter_shares_columns(const ProjParams& p)
     // 3.1 rays per slice and 2.1 planes (512x512x128, 45 views of 800 x 800), 1.12
     // at 1.5 and 2.1 (256x256x64), 1.0 at 2.6 and 1.7 (126x126x49), but 0.9 at
     // 1.3 and 5.8 (74x74x39), 0.7 at 1.4 and 3.7 (146x146x140).
-    const double pitch = p.piso * p.dpn / p.H;
-    const double planes = 32.0 * p.piso * p.dpn / 2.0 / p.sad * p.s / p.step;
-    return march_shares_columns(p) && p.step >= 1.4 * pitch && planes <= 2.5;
+    const ColumnShape c = column_shape(p);
+    return rays_share_slices(c) && c.rays >= 1.4 && c.planes <= 2.5;
 }
 
 cudaError_t launch_forward(const ForwardArgs& a, cudaStream_t st)
