@@ -2349,12 +2349,17 @@ bool scatter_shares_columns(const ProjParams& p)
 {
     // The scatter's own line: a ray's walk of the chunks in which it meets a z
     // plane costs more than the forward's, so it also asks that the steepest
-    // ray meet few of them per batch of steps.  B200, columns / walk: 1.66 at
-    // 3.1 rays per slice and 2.1 planes (512x512x128, 45 views of 800 x 800), 1.12
-    // at 1.5 and 2.1 (256x256x64), 1.0 at 2.6 and 1.7 (126x126x49), but 0.9 at
-    // 1.3 and 5.8 (74x74x39), 0.7 at 1.4 and 3.7 (146x146x140).
+    // ray meet few of them per batch of steps, and the more of them the rays
+    // inside the slab meet, the more rays to a slice.  B200, times by shared columns /
+    // walked: 1.66 at 3.1 rays and 2.1 planes (512x512x128, 45 views of 800 x 800), 0.9
+    // at 1.3 and 5.8 (74x74x39), 0.7 at 1.4 and 3.7 (146x146x140); by the planes
+    // inside the slab, large volumes 1.08 at 1.0 and 1.45 rays (256x256x65), 0.84 at
+    // 2.0 and 1.45, 0.92 and 1.8, 1.07 and 2.4 (215x215x110), small ones 0.98 at 0.7
+    // and 1.45, 1.15 and 1.8 (128x128x26), 0.85 at 1.8 and 1.8, 0.97 and 2.4, 1.08
+    // and 3.5 (96x96x44).
     const ColumnShape c = column_shape(p);
-    return rays_share_slices(c) && c.rays >= 1.4 && c.planes <= 2.5;
+    const double least = fmax(1.4, c.small ? 1.7 + 0.9 * (c.inside - 0.8) : 1.4 + 0.75 * (c.inside - 1.2));
+    return rays_share_slices(c) && c.planes <= 2.5 && c.rays >= least;
 }
 
 cudaError_t launch_forward(const ForwardArgs& a, cudaStream_t st)
