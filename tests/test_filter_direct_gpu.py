@@ -25,3 +25,24 @@ def test_direct_filter_matches_fp64(cuda, V, H, W):
     h = np.abs(O.const_map(W, consts)) + abs(O.filter_coeff(W, consts)) * np.eye(W)
     bound = (W + 10) * 2.0 ** -24 * (np.abs(np.log(proj.astype(np.float64))) @ h.T)
     assert (np.abs(got - ref) <= bound).all()
+
+
+@pytest.mark.parametrize("V,H,W", [(40, 250, 200), (48, 200, 256), (40, 250, 193)])
+def test_staged_rows_serve_every_column_pass(cuda, V, H, W):
+    """Two column passes a block over rows that stay in shared memory (193 to 256
+    columns, more row blocks than SMs): each row filtered as in a stack that
+    gives every pass a block of its own."""
+    import torch
+    assert V * H > 64 * 148
+    proj = torch.rand((V, H, W), generator=torch.Generator().manual_seed(W)).mul_(0.98).add_(0.02).cuda()
+    ang, xs, ys = np.deg2rad(np.arange(V) * 360.0 / V), np.full(V, 2.0), np.zeros(V)
+    geom = dict(H=H, W=W, N=8, Z=2, zstart=-1, step=0.5, scale=0.4)
+    got = Fdk(FdkGeometry(V=V, **geom), ang, xs, ys).filter(proj)
+    few = Fdk(FdkGeometry(V=8, **geom), ang[:8], xs[:8], ys[:8])
+    for v in range(0, V, 8):
+        assert torch.equal(got[v:v + 8], few.filter(proj[v:v + 8].contiguous()))
+    ref = O.filter_sinogram(proj[:2].cpu().numpy(), xs[:2], ys[:2], O.fdk_consts(few.geom.piso), mode=1)
+    consts = O.fdk_consts(few.geom.piso)
+    h = np.abs(O.const_map(W, consts)) + abs(O.filter_coeff(W, consts)) * np.eye(W)
+    bound = (W + 10) * 2.0 ** -24 * (np.abs(np.log(proj[:2].cpu().numpy().astype(np.float64))) @ h.T)
+    assert (np.abs(got[:2].cpu().numpy() - ref) <= bound).all()

@@ -25,6 +25,20 @@ def test_lengthproj_matches_oracle(cuda, ite, xshift, views):
     assert np.array_equal(dev, ref)
 
 
+@pytest.mark.parametrize("N,Z", [(24, 11),     # two slices a thread, one past the slab
+                                 (320, 19),    # four, one past
+                                 (320, 20), (320, 23), (320, 24)])  # four; eight, one past; eight
+def test_lengthproj_slices_a_thread(cuda, N, Z):
+    from tests.cases import proj_case
+    blocks = -(-N // 32) * -(-N // 8) * -(-Z // 8)  # of eight slices: the rule's own terms
+    assert (blocks >= 4 * 148) == (N == 320) and (-Z % 8 > Z // 8) == (Z in (11, 19, 20))
+    g, tabs, _, _ = proj_case("water", N=N, Z=Z, s=25.6 / N, step=0.25, V=3, W=40, H=32)
+    proj = np.random.default_rng(Z).integers(20000, 65000, size=(g.V, g.H, g.W)).astype(np.uint16)
+    got = Projector(g, *tabs).lengthproj(proj)
+    ref = O.lengthproj(g, tabs, proj)
+    assert np.abs(ref).max() > 0 and np.array_equal(got, ref), np.abs(got - ref).max()
+
+
 def test_lengthproj_reference_named_entry_point(cuda):
     import ctypes as C
     g, tabs, proj = ir_case(seed=9)
