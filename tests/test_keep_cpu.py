@@ -16,3 +16,18 @@ def test_keep_asks_for_free_memory_only_above_the_small_share(monkeypatch):
     assert autograd._keep(1 << 30, None) and len(asked) == 1
     assert not autograd._keep((1 << 30) + 1, None) and len(asked) == 2
     assert not autograd._keep(1, 0) and autograd._keep(1, 1) and len(asked) == 2
+
+
+def test_keep_on_a_nearly_full_device(monkeypatch):
+    """Small path integrals are not held where a quarter of the free memory is
+    less, unless torch holds the step's memory already."""
+    total, asked, held = 180 << 30, [], {}
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: SimpleNamespace(total_memory=total))
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda: asked.append(1) or (16 << 20, total))
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda: held)
+    n = 100 << 20
+    assert not autograd._keep(n, None) and len(asked) == 1  # nothing held: the allocator has not run
+    held.update(reserved_bytes={"all": {"current": 10 * n}}, allocated_bytes={"all": {"current": 7 * n}})
+    assert autograd._keep(n, None, 2 * n) and len(asked) == 1
+    assert not autograd._keep(n, None, 2 * n + 1) and len(asked) == 2

@@ -23,17 +23,30 @@ from .projector import Projector, _volume_key
 # when they take at most a quarter of the device's free memory (11 GB for 720
 # views of 800 x 800 is kept on a 180 GB GPU).
 KEEP_LIMIT = None
-# Asking the driver for the free memory takes 69 us to 2.5 ms on a shared node, a
-# fifth of a small step or more (56x56x9, 36 views of 30 x 46: 347 us, 240
-# without), so path integrals below this share of
-# the device's memory are kept without asking, and re-marched only if their
-# allocation fails.
-SMALL_SHARE = 1024
+# Asking the driver for the free memory takes 69 us to several ms on a shared
+# node, a fifth of a small step or more (56x56x9, 36 views of 30 x 46: 347 us,
+# 240 without).  It is not asked where the answer cannot matter: for path
+# integrals below this share of the device's memory (1.4 MB of 180 GB, less than
+# the 2 MB in which torch takes device memory), and where torch already holds
+# the memory of the whole step free, as from the second step of a loop on
+# (looking that up takes 11 us).
+SMALL_SHARE = 1 << 17
 
 
-def _keep(nbytes: int, keep_limit) -> bool:
+def _held_free() -> int:
+    """Bytes that torch's allocator holds free on the current device."""
+    s = torch.cuda.memory_stats_as_nested_dict()
+    now = [s.get(k, {}).get("all", {}).get("current", 0) for k in ("reserved_bytes", "allocated_bytes")]
+    return now[0] - now[1]
+
+
+def _keep(nbytes: int, keep_limit, rest: int = 0) -> bool:
+    """Whether to keep ``nbytes`` of path integrals; ``rest``: bytes that the
+    step allocates after them."""
     if keep_limit is None:
         if nbytes <= torch.cuda.get_device_properties(torch.cuda.current_device()).total_memory // SMALL_SHARE:
+            return True
+        if nbytes + rest <= _held_free():
             return True
         free, _ = torch.cuda.mem_get_info()
         return nbytes <= free // 4
@@ -50,7 +63,8 @@ class _MbfpaProject(torch.autograd.Function):
         g = projector.geom
         out = torch.empty((g.V, g.H, g.W), dtype=torch.float32, device="cuda")
         L = None
-        if _keep(g.V * g.H * g.W * g.nmat * 4, keep_limit):
+        # after them: the gradient, and a residual and its square of the projections' size
+        if _keep(g.V * g.H * g.W * g.nmat * 4, keep_limit, 4 * vol.numel() + 2 * 4 * out.numel()):
             try:
                 L = torch.empty((g.V, g.H, g.W, g.nmat), dtype=torch.float32, device="cuda")
             except torch.OutOfMemoryError:
@@ -85,8 +99,9 @@ class _MbfpaProject(torch.autograd.Function):
 def project(volumes: torch.Tensor, projector: Projector, keep_limit=KEEP_LIMIT) -> torch.Tensor:
     """Differentiable spectral forward projection of float element volumes.
     The per-ray path integrals are kept for the backward pass when they fit
-    in ``keep_limit`` bytes (0: always re-march; None: a quarter of the free
-    device memory)."""
+    in ``keep_limit`` bytes (0: always re-march; None: in a quarter of the free
+    device memory, or together with the rest of the step in memory that torch
+    already holds)."""
     return _MbfpaProject.apply(volumes, projector, keep_limit)
 
 
