@@ -154,3 +154,25 @@ def test_more_tiles_than_a_grid_holds(cuda):
     b.forward(use_graph=False)
     for p, o in zip(ps, outs):
         assert torch.equal(o, p.forward())
+
+
+def test_tuned_choices_are_kept_apart_by_kernel(cuda, monkeypatch, tmp_path):
+    """Projectors and batches of equal sizes, walked or by shared columns, of
+    uint16 or float volumes: none takes a choice that was timed for another."""
+    file = tmp_path / "tuned"
+    monkeypatch.setenv("VCBCT_TUNE_CACHE", str(file))
+    seen = 0
+    for step in (0.2, 0.6):
+        for f32 in (False, True):
+            g, tabs, vol, _ = proj_case("random", seed=1, N=31, Z=7, V=3, W=21, H=45, step=step)
+            mu, pdf = spectrum()
+            p = Projector(g, *tabs)
+            p.set_spectrum(mu, pdf, 1000.0)
+            p.load_volume_f32(vol.astype(np.float32)) if f32 else p.load_volume(vol)
+            b = Batch()
+            b.add(p)
+            for again in (0, 1):
+                p.autotune()
+                b.autotune()
+                assert len(file.read_text().splitlines()) == seen + 2
+            seen += 2

@@ -1099,8 +1099,11 @@ extern "C" int vcbct_batch_forward(vcbct_batch* b, int use_graph, void* stream)
 //
 // Launch shapes are picked by timing the candidates on the caller's data:
 // columns per block (warps per block) for the plain and the batched forward
-// projection.  Results are kept per geometry signature in memory and, when
-// VCBCT_TUNE_CACHE names a file, in that file ("signature value" lines).
+// projection.  Results are kept per signature in memory and, when
+// VCBCT_TUNE_CACHE names a file, in that file ("signature value" lines).  A
+// signature holds what picks the kernel and its work: the sizes, the elements
+// and bins, whether the rays share columns, the form of the volume, and the
+// generation of the kernels, so that a choice made for others is not taken.
 
 namespace {
 std::mutex g_tune_mu;
@@ -1139,6 +1142,18 @@ std::string device_tag()
     return n;
 }
 
+constexpr const char* kKernels = "2";  // counts up when the forward kernels' speeds change
+
+std::string tune_key(const vcbct_projector* p)
+{
+    const auto& g = p->g;
+    std::ostringstream key;
+    key << g.recon_size << "x" << g.recon_slices << ":" << g.proj_width << "x" << g.proj_height << "x" << g.n_views << ":"
+        << g.num_material << ":" << p->NE << ":" << (march_shares_columns(p->pp) ? "columns" : "walk") << ":"
+        << (p->have_u16 ? "u16" : "f32");
+    return key.str();
+}
+
 template <class F>
 float time_ms(F f, cudaStream_t st, int reps)
 {
@@ -1163,11 +1178,8 @@ extern "C" int vcbct_projector_autotune(vcbct_projector* p, float* d_out, void* 
     if (!p || !d_out) return fail(VCBCT_ERR_ARG, "NULL argument");
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_load();
-    const auto& g = p->g;
-    std::ostringstream key;
-    key << "fwd:" << device_tag() << ":" << g.recon_size << "x" << g.recon_slices << ":" << g.proj_width << "x"
-        << g.proj_height << "x" << g.n_views << ":" << g.num_material << ":" << p->NE;
-    auto it = g_tune.find(key.str());
+    const std::string key = "fwd" + std::string(kKernels) + ":" + device_tag() + ":" + tune_key(p);
+    auto it = g_tune.find(key);
     if (it == g_tune.end()) {
         cudaStream_t st = (cudaStream_t)stream;
         float best = 1e30f;
@@ -1180,7 +1192,7 @@ extern "C" int vcbct_projector_autotune(vcbct_projector* p, float* d_out, void* 
                 bestc = c;
             }
         }
-        tune_store(key.str(), bestc);
+        tune_store(key, bestc);
         p->cols_per_block = bestc;
     } else {
         p->cols_per_block = it->second;
@@ -1195,10 +1207,8 @@ extern "C" int vcbct_batch_autotune(vcbct_batch* b, void* stream, int* chosen)
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_load();
     std::ostringstream key;
-    key << "batch:" << device_tag() << ":" << b->proj.size();
-    for (auto* p : b->proj)
-        key << ":" << p->g.recon_size << "x" << p->g.recon_slices << "x" << p->g.n_views << "x" << p->g.proj_width
-            << "x" << p->g.proj_height;
+    key << "batch" << kKernels << ":" << device_tag() << ":" << b->proj.size();
+    for (auto* p : b->proj) key << ":" << tune_key(p);
     auto it = g_tune.find(key.str());
     int bestc = b->cols_per_block + 100 * b->strategy;
     if (it == g_tune.end()) {
