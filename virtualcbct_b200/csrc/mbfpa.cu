@@ -2035,12 +2035,14 @@ __device__ __forceinline__ void set_form(int* form, int f)
 }
 
 // 64 x by 32 z of one y: bound by memory (2 nmat bytes read and 16 written a
-// voxel).  A thread reads two neighbouring x of an element row at a time (one
-// 4-byte load where rows are 4-byte aligned: PAIR), all elements in flight,
-// and packs their records in registers; shared memory only turns the order from
-// x to z fastest, 16 bytes a lane without bank conflicts (the two x of a pair
-// lie 32 columns apart).  512x512x200 x 6: 0.74 ms as floats through
-// 2-byte loads, 0.34 ms now (0.22 at the copy rate).
+// voxel).  A thread reads two x of an element row at a time, all elements in
+// flight, and packs their records in registers; shared memory only turns the
+// order from x to z fastest, 16 bytes a lane without bank conflicts (a thread's
+// two x lie 32 columns apart in it).  Where rows are 4-byte aligned the two are
+// neighbours, one load (PAIR): 512x512x200 x 6 0.74 ms as floats through 2-byte
+// loads, 0.34 ms now (0.22 at the copy rate).  Elsewhere they are 32 apart, so that
+// either load of a warp reads one run, and neither waits behind a branch of its
+// own: 203x203x77 0.069 -> 0.047 ms, 511x511x100 0.38 -> 0.25.
 template <bool PAIR>
 __global__ void __launch_bounds__(256) pack_u16_kernel(const uint16_t* __restrict__ src, int N, int nz, int zoff, int Z,
                                                        int nmat, uint4* __restrict__ dst, int* form)
@@ -2049,18 +2051,22 @@ __global__ void __launch_bounds__(256) pack_u16_kernel(const uint16_t* __restric
     __shared__ uint4 tile[64][33];
     const int x0 = blockIdx.x * 64, y = blockIdx.y, z0 = blockIdx.z * 32;
     const size_t NN = (size_t)N * N;
-    const int l = threadIdx.x, x = x0 + 2 * l;
+    const int l = threadIdx.x, x = x0 + (PAIR ? 2 * l : l);
 #pragma unroll 2
     for (int zz = threadIdx.y; zz < 32; zz += 8) {
         const int z = z0 + zz;
+        const uint16_t* q = src + (size_t)z * nmat * NN + (size_t)y * N + x;
+        const bool in = z < nz && x < N, in2 = z < nz && x + 32 < N;
         uint32_t w[8];
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             w[m] = 0u;
-            if (m < nmat && z < nz && x < N) {
-                const uint16_t* q = src + ((size_t)z * nmat + m) * NN + (size_t)y * N + x;
-                if (PAIR) w[m] = __ldg(reinterpret_cast<const uint32_t*>(q));
-                else w[m] = (uint32_t)__ldg(q) | (x + 1 < N ? (uint32_t)__ldg(q + 1) << 16 : 0u);
+            if (PAIR) {
+                if (m < nmat && in) w[m] = __ldg(reinterpret_cast<const uint32_t*>(q + m * NN));
+            } else {
+                const uint32_t lo = m < nmat && in ? __ldg(q + m * NN) : 0u;
+                const uint32_t hi = m < nmat && in2 ? __ldg(q + m * NN + 32) : 0u;
+                w[m] = lo | hi << 16;
             }
         }
         tile[l][zz] = make_uint4(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410),
@@ -2073,7 +2079,7 @@ __global__ void __launch_bounds__(256) pack_u16_kernel(const uint16_t* __restric
     if (z >= nz) return;
     for (int xx = threadIdx.y; xx < 64; xx += 8) {
         if (x0 + xx >= N) break;
-        dst[((size_t)y * N + x0 + xx) * Z + zoff + z] = tile[(xx >> 1) + 32 * (xx & 1)][l];
+        dst[((size_t)y * N + x0 + xx) * Z + zoff + z] = tile[PAIR ? (xx >> 1) + 32 * (xx & 1) : xx][l];
     }
 }
 
