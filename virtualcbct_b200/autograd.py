@@ -25,12 +25,12 @@ from .projector import Projector, _volume_key
 KEEP_LIMIT = None
 # Asking the driver for the free memory takes 69 us to several ms on a shared
 # node, a fifth of a small step or more (56x56x9, 36 views of 30 x 46: 347 us,
-# 240 without).  It is not asked where the answer cannot matter: for path
-# integrals below this share of the device's memory (1.4 MB of 180 GB, less than
-# the 2 MB in which torch takes device memory), and where torch already holds
-# the memory of the whole step free, as from the second step of a loop on
-# (looking that up takes 11 us).
-SMALL_SHARE = 1 << 17
+# 240 without).  It is not asked for path integrals below this share of the
+# device's memory (22 MB of 180 GB, about the unit of 20 MB in which torch takes
+# device memory), nor where torch already holds the memory of the whole step
+# free, as from the second step of a loop on (looking that up takes 11 us, 3 to
+# 7 % of steps of 0.4 ms: hence the share).
+SMALL_SHARE = 1 << 13
 
 
 def _held_free() -> int:
