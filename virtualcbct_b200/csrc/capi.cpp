@@ -168,7 +168,7 @@ extern "C" int vcbct_projector_create(const vcbct_proj_geometry* g, const double
     // from 360 views, 3.38 / 3.55 ms at 203x203x77 from 91) while the GPU
     // still gets three blocks per SM
     if (march_shares_columns(p->pp) &&
-        (long long)((g->proj_width + 7) / 8) * g->n_views * ((g->proj_height + 31) / 32) >= 3 * 148)
+        (long long)((g->proj_width + 7) / 8) * g->n_views * ((g->proj_height + 31) / 32) >= 3 * kSMs)
         p->cols_per_block = 8;
     if (const char* c = std::getenv("VCBCT_COLS_PER_BLOCK")) {
         int v = std::atoi(c);

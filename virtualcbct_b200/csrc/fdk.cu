@@ -208,7 +208,8 @@ __device__ __forceinline__ void filter_pass(const FilterArgs& a, int r0, int n0,
     }
 }
 
-// MAXTN: the widest pass; narrow passes leave registers for twice the blocks.
+// MAXTN: the widest pass; narrow passes leave registers for twice the blocks (of
+// which three fit where a block stages 256 columns, four up to 192).
 template <int MAXTN>
 __global__ void __launch_bounds__(256, MAXTN <= 2 ? 4 : 2) filter_direct_kernel(const __grid_constant__ FilterArgs a)
 {
@@ -576,7 +577,7 @@ cudaError_t launch_filter_direct(const float* proj, float* out, const float* hT,
     // One block makes every column pass of its rows, or a part of them where
     // the rows alone would not fill the GPU (two blocks an SM); narrower
     // passes where that is still so.
-    const int rows = (M + FT_M - 1) / FT_M, want = std::max(1, 2 * 148 / rows);
+    const int rows = (M + FT_M - 1) / FT_M, want = std::max(1, 2 * kSMs / rows);
     if (a.npass < want) a.npass = std::min(a.groups, want);
     // (g does not stay staged from pass to pass beyond FT_CHUNK columns: then
     // every pass is a block of its own, and the last wave is shorter)
@@ -625,22 +626,25 @@ cudaError_t launch_backproject(const FdkParams& f, const BpView* d_views, const 
     const bool sv = table_bytes + mask_bytes <= 48 * 1024;
     const size_t smem = mask_bytes + (sv ? table_bytes : 0);
     // resident blocks per SM (the register cap): VCBCT_BP_MIN_BLOCKS by
-    // default, 5 or 6 through the environment variable of the same name
+    // default, 5 or 6 through the environment variable of the same name where
+    // a thread makes a whole slice block
     int minb = VCBCT_BP_MIN_BLOCKS;
     if (const char* e = std::getenv("VCBCT_BP_MIN_BLOCKS")) minb = std::atoi(e) == 6 ? 6 : 5;
     auto launch = [&](auto zs) {
         constexpr int ZS = decltype(zs)::value;
         const dim3 gp(grid.x, grid.y, grid.z * (ZB / ZS));
-        auto k5 = sv ? backproject_kernel<ZB, ZS, 5, true> : backproject_kernel<ZB, ZS, 5, false>;
-        auto k6 = sv ? backproject_kernel<ZB, ZS, 6, true> : backproject_kernel<ZB, ZS, 6, false>;
-        (minb == 5 ? k5 : k6)<<<gp, block, smem, st>>>(f, k, d_views, filt, vol_f32, vol_i16, keep);
+        auto kernel = sv ? backproject_kernel<ZB, ZS, 5, true> : backproject_kernel<ZB, ZS, 5, false>;
+        if constexpr (ZS == ZB)
+            if (minb == 6) kernel = sv ? backproject_kernel<ZB, ZS, 6, true> : backproject_kernel<ZB, ZS, 6, false>;
+        kernel<<<gp, block, smem, st>>>(f, k, d_views, filt, vol_f32, vol_i16, keep);
     };
     // Threads of fewer slices repeat the column's set-up, which is free while
     // SM slots (five an SM) stand idle.  Slices a thread 8 / 4 / 2, us on a B200:
     // 396 blocks (95x95x84) 151 / 154 / 154, 340 blocks 372 / 407 / 451, 231
     // blocks (86x86x51) 32 / 21 / 21, 190 blocks 33 / 25 / 21, 120 blocks
     // (80x80x27, 224 views of 793 x 720) 489 / 327 / 220, 128 blocks (58x58x64)
-    // 341 / 249 / 295.
+    // 341 / 249 / 295: two slices are not the best of every volume below 200
+    // blocks, but better than eight.
     if (nblocks >= 300) launch(std::integral_constant<int, ZB>{});
     else if (nblocks >= 200) launch(std::integral_constant<int, ZB / 2>{});
     else launch(std::integral_constant<int, ZB / 4>{});

@@ -20,6 +20,8 @@ int cuda_fail(cudaError_t e, const char* what);
         if (e__ != cudaSuccess) return ::vcbct::cuda_fail(e__, #call); \
     } while (0)
 
+constexpr int kSMs = 148;  // of a B200, the only GPU this library is built for
+
 // A launch whose blocks take more than 48 KB of dynamic shared memory needs its
 // kernel's limit raised.  The limit is the kernel's (on a device), shared by
 // every host thread and by launches prepared long before, so it is only ever

@@ -213,7 +213,7 @@ cudaError_t launch_lengthproj(const LpParams& q, const ViewGeom* d_views, int v0
         return dim3((unsigned)((q.N + 31) / 32), (unsigned)((q.N + 7) / 8), (unsigned)((q.Z + zb - 1) / zb));
     };
     const dim3 g8 = grid(8);
-    if ((long long)g8.x * g8.y * g8.z < 4 * 148)
+    if ((long long)g8.x * g8.y * g8.z < 4 * kSMs)
         lengthproj_kernel<2><<<grid(2), block, 0, st>>>(q, vw, v0, nv, d_proj, d_npf);
     else if (8 * (int)g8.z - q.Z > q.Z / 8)
         lengthproj_kernel<4><<<grid(4), block, 0, st>>>(q, vw, v0, nv, d_proj, d_npf);
