@@ -475,7 +475,8 @@ def iterative_section(stream):
     ir_bytes = 14.0 * nvox  # short before + float npf, npf_re, out (neighbours from cache)
     res = {"workload": "512x512x100, 36 views of 400x400 uint16",
            "lengthproj_ms": lp, "lengthproj_gvox_views_s": nvox * g.V / (lp * 1e-3) / 1e9,
-           "lengthproj_bound": "fp64 (the reference's double arithmetic, about 8 divisions per voxel-view)",
+           "lengthproj_bound": "fp64 (the reference's double arithmetic: a square root and two quotients per voxel-view, "
+                              "six divisions per column of slices and view)",
            "ir_update_ms": ir, "ir_update_gvox_s": nvox / (ir * 1e-3) / 1e9,
            "ir_update_roofline": {"bound": "hbm", "achieved": ir_bytes / (ir * 1e-3) / 1e9, "peak": peak,
                                   "unit": "GB/s", "frac": ir_bytes / (ir * 1e-3) / 1e9 / peak,

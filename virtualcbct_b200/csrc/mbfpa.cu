@@ -28,7 +28,8 @@
 // the batch kernels (persistent work queue, flat tile list), the adjoint
 // (per-ray spectral derivative, then the same segments scattered into
 // z-fastest planes of element groups, summed per slice first where rays share
-// one, optionally restricted to a strip of volume rows), and the volume / gradient re-layout kernels.
+// one, optionally restricted to a strip of volume rows), and the volume /
+// gradient re-layout kernels.
 #include "internal.h"
 #include "noise.cuh"
 
@@ -1514,8 +1515,8 @@ __device__ __forceinline__ f32x2 exp2_2(f32x2 x)
 // under the floor, or one that is not finite (a path integral that only its
 // scaling takes beyond the largest float), is done again with expf and L as it is.
 // Asking every bin instead did most sums of a body twice: 10 keV bins behind
-// 20 cm of water are below 2^-126 (48 phantoms of 64x64xZ: 0.321 -> 0.284 ms; 256x256x100, 60 views of
-// 200 x 200: 1.54 -> 1.44).
+// 20 cm of water are below 2^-126 (48 phantoms of 64x64xZ: 0.321 -> 0.284 ms;
+// 256x256x100, 60 views of 200 x 200: 1.54 -> 1.44).
 template <int M>
 __device__ __forceinline__ float spectral_sum(const SpecPair<M>* s_sp, int NE, const float* L)
 {
@@ -1738,12 +1739,13 @@ size_t block_smem(int NE, int cpb, bool sums, bool col, size_t tab = sizeof(ColT
 // across views).
 // Register cap of the forward kernel: minimum resident 256-thread blocks per
 // SM.  The walk is bound by the latency of its gathers; with one of them in
-// flight behind the sums (PIPE), 4 blocks (64 registers, 32 warps) beat both
-// fewer warps and fewer registers (448x448x120 floats, 100 x 100 x 60 views: 1.44
-// ms, 5 blocks 1.40, 3 blocks 1.69, 6 without PIPE 1.55; 64x64x16, 32 x 32 x 60
-// views: 0.049, 0.054, 0.045, 0.062).  The column march has more state and more
-// loads in flight per warp: 3 blocks (80 registers, 24 warps) 32.1 ms on
-// 512x512x200 from 360 views, 4 blocks 35.9, 2 blocks 36.6.
+// flight behind the sums (PIPE), 4 blocks (64 registers, of which few spill: 44 to
+// 84 bytes; 32 warps) are never far from the best: 448x448x120 floats, 100 x
+// 100 x 60 views 1.44 ms, 5 blocks 1.40, 3 blocks 1.69, 6 without PIPE 1.55;
+// 64x64x16, 32 x 32 x 60 views 0.049, 0.054, 0.045, 0.062; 64 phantoms of
+// 128x128xZ, floats, flat 5.9, 5.9, 6.6 and 6.9.  The column march has more state
+// and more loads in flight per warp: 3 blocks (80 registers, 24 warps) 32.1 ms
+// on 512x512x200 from 360 views, 4 blocks 35.9, 2 blocks 36.6.
 constexpr int fwd_min_blocks(int mode) { return mode == kWalk ? 4 : 3; }
 template <int M, bool COUNT, int MODE, bool U16>
 __global__ void __launch_bounds__(256, fwd_min_blocks(MODE)) forward_kernel(const __grid_constant__ ForwardArgs a)
@@ -1899,8 +1901,10 @@ __global__ void __launch_bounds__(256, 5) persistent_batch_kernel(const __grid_c
 }
 
 // Register cap of the adjoint (minimum resident 256-thread blocks per SM):
-// 3 (80 registers) and 4 (64) measured within 1.5 % on B200, 5 (48) 15 %
-// slower; 3 is kept.
+// 512x512x128 floats, 45 views of 800 x 800 by shared columns, with kept path
+// integrals / re-marching them: 3 blocks (80 registers) 21.9 / 40.0 ms, 4 (64) 22.8 /
+// 50.2, 5 (48) 33.6 / 65.8, 2 25.3 / 43.6; 300x300x100, 40 views of 160 x 150 on
+// their own: 1.71 / 3.15, 1.70 / 2.96, 1.88 / 3.02, 1.97 / 3.80.
 #ifndef VCBCT_ADJ_MIN_BLOCKS
 #define VCBCT_ADJ_MIN_BLOCKS 3
 #endif
@@ -2142,7 +2146,6 @@ __global__ void __launch_bounds__(256) pack_f32_kernel(const float* __restrict__
     }
 }
 
-// packed float records -> [Z][nmat][N][N], accumulated (+=).
 // element planes [nmat][(y*N + x)*Z + z] -> [Z][nmat][N][N], accumulated (+=).
 // grid (ceil(N/32), N, ceil(Z/32) * nmat), block (32, 8): a 32 x 32 (x, z)
 // tile of one plane through shared memory.
