@@ -505,8 +505,7 @@ struct PairSums {
 template <int M, bool PIPE = false>
 struct AccumU16 : PairSums<M> {
     const uint4* __restrict__ vol;
-    unsigned nseg;
-    __device__ __forceinline__ AccumU16(const uint4* v, float* ls) : vol(v), nseg(0u)
+    __device__ __forceinline__ AccumU16(const uint4* v, float* ls) : vol(v)
     {
         this->Ls = ls;
         this->clear();
@@ -547,7 +546,6 @@ struct AccumU16 : PairSums<M> {
         } else {
             add(this->P2, load(idx), f2pack(len, len));
         }
-        nseg++;
     }
     __device__ __forceinline__ void drain() { add(this->P2, pend, f2pack(plen, plen)); }
     // before the pair sums are folded
@@ -570,7 +568,6 @@ struct AccumU16 : PairSums<M> {
             f2unpack(u16pair(w[i / 2]), a, b);
             this->Ls[i * ls_stride()] = fmaf((i & 1) ? b : a, len, this->Ls[i * ls_stride()]);
         }
-        nseg++;
     }
 };
 
@@ -578,8 +575,7 @@ template <int M, bool PIPE = false>
 struct AccumF32 : PairSums<M> {
     using Base = PairSums<M>;
     const uint4* __restrict__ vol;
-    unsigned nseg;
-    __device__ __forceinline__ AccumF32(const uint4* v, float* ls) : vol(v), nseg(0u)
+    __device__ __forceinline__ AccumF32(const uint4* v, float* ls) : vol(v)
     {
         this->Ls = ls;
         this->clear();
@@ -637,7 +633,6 @@ struct AccumF32 : PairSums<M> {
         } else {
             add(this->P2, load(idx), f2pack(len, len));
         }
-        nseg++;
     }
     __device__ __forceinline__ void drain() { add(this->P2, pend, f2pack(plen, plen)); }
     // before the pair sums are folded
@@ -657,7 +652,6 @@ struct AccumF32 : PairSums<M> {
         for (int i = 0; i < M; i++) {
             this->Ls[i * ls_stride()] = fmaf(__ldg(p + i), len, this->Ls[i * ls_stride()]);
         }
-        nseg++;
     }
 };
 
@@ -1635,18 +1629,29 @@ __device__ __forceinline__ void ray_integrals(const ProjParams& P, const RayPlan
 
 __device__ __forceinline__ bool is_u16(const VolRef& v) { return (v.form ? *v.form : v.expect) == kFormU16; }
 
-// Path integrals of one ray; returns the segments the lane visited (kWalk:
-// all of them).
+// Counts the segments of a ray that walks; reads no volume.
+struct SegmentCount {
+    unsigned nseg = 0u;
+    float lt;
+    __device__ __forceinline__ void operator()(int, float) { nseg++; }
+    __device__ __forceinline__ void first(int, float) { nseg++; }
+    __device__ __forceinline__ void lanes(bool p, int, float) { nseg += p; }
+    __device__ __forceinline__ void clear() {}
+    __device__ __forceinline__ void settle() {}
+    __device__ __forceinline__ void fold() {}
+    __device__ __forceinline__ void zero_L() {}
+};
+
+// Path integrals of one ray.
 template <int M, int MODE, bool U16>
-__device__ __forceinline__ unsigned ray_path(const VolRef& vol, const ProjParams& P, const RayPlan& R, bool act, int Klo,
-                                             int Khi, IvRec* wbuf, float* s_L, ColTab<M>* tab, float (&L)[M])
+__device__ __forceinline__ void ray_path(const VolRef& vol, const ProjParams& P, const RayPlan& R, bool act, int Klo,
+                                         int Khi, IvRec* wbuf, float* s_L, ColTab<M>* tab, float (&L)[M])
 {
     typedef std::conditional_t<U16, AccumU16<M, MODE == kWalk>, AccumF32<M, MODE == kWalk>> Acc;
     Acc acc(static_cast<const uint4*>(vol.rec), s_L);
     ray_integrals<Acc, M, MODE>(P, R, act, Klo, Khi, wbuf, acc, tab);
 #pragma unroll
     for (int i = 0; i < M; i++) L[i] = acc.Lget(i);
-    return acc.nseg;
 }
 
 // One work tile of the forward projection: detector columns
@@ -1671,18 +1676,20 @@ __device__ __forceinline__ void forward_tile_of(const ForwardArgs& a, const Spec
     int Klo, Khi;
     warp_range(R, valid, Klo, Khi);
 
+    if constexpr (COUNT) {
+        SegmentCount n;
+        ray_integrals<SegmentCount, M, MODE>(P, R, valid, Klo, Khi, wbuf, n, nullptr);
+        const unsigned tot = __reduce_add_sync(0xffffffffu, valid ? n.nseg : 0u);
+        if (lane == 0 && tot) atomicAdd(a.seg_count, (unsigned long long)tot);
+        return;
+    }
     float L[M];
-    unsigned nseg = 0;
     float* s_L = reinterpret_cast<float*>(s_iv + blockDim.y * kSlots) + threadIdx.y * 32 + lane;
     ColTab<M>* tab = nullptr;
     if (MODE == kColumns)
         tab = reinterpret_cast<ColTab<M>*>(reinterpret_cast<float*>(s_iv + blockDim.y * kSlots) +
                                            M * 32 * blockDim.y) + threadIdx.y;
-    nseg = ray_path<M, MODE, U16>(a.vol, P, R, valid, Klo, Khi, wbuf, s_L, tab, L);
-    if (COUNT) {
-        unsigned tot = __reduce_add_sync(0xffffffffu, valid ? nseg : 0u);
-        if (lane == 0 && tot) atomicAdd(a.seg_count, (unsigned long long)tot);
-    }
+    ray_path<M, MODE, U16>(a.vol, P, R, valid, Klo, Khi, wbuf, s_L, tab, L);
     if (!valid) return;
     const size_t o = ((size_t)v * P.H + (P.H - 1 - j)) * P.W + jj;
     if (a.L_out) {
@@ -1714,7 +1721,8 @@ template <int M, bool COUNT, int MODE, bool U16>
 __device__ __forceinline__ void forward_tile(const ForwardArgs& a, const SpecPair<M>* s_sp, IvRec* s_iv, int v,
                                              int rowt, int colb)
 {
-    if (is_u16(a.vol) == U16) forward_tile_of<M, COUNT, MODE, U16>(a, s_sp, s_iv, v, rowt, colb);
+    if constexpr (COUNT) forward_tile_of<M, COUNT, MODE, U16>(a, s_sp, s_iv, v, rowt, colb);
+    else if (is_u16(a.vol) == U16) forward_tile_of<M, COUNT, MODE, U16>(a, s_sp, s_iv, v, rowt, colb);
     else forward_tile_other<M, COUNT, MODE, !U16>(a, s_sp, s_iv, v, rowt, colb);
 }
 
@@ -2373,11 +2381,11 @@ bool scatter_shares_columns(const ProjParams& p)
 
 cudaError_t launch_forward(const ForwardArgs& a, cudaStream_t st)
 {
+    if (a.seg_count) return launch_fwd_t<6, true, kWalk, false>(a, st);
     const bool u16 = a.vol.expect == kFormU16;
     auto launch = [&](auto m, auto u) {
         constexpr int M = decltype(m)::value;
         constexpr bool U = decltype(u)::value;
-        if (a.seg_count) return launch_fwd_t<M, true, kWalk, U>(a, st);
         if (a.columns) return launch_fwd_t<M, false, kColumns, U>(a, st);
         return launch_fwd_t<M, false, kWalk, U>(a, st);
     };
